@@ -2102,6 +2102,53 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: to
     )
 
 
+CHUNKED_TOKENS = 64  # tokens a chunk (csrc/chunked_recurrence.cu)
+# Where the line lies (16 heads of 128 columns; us a chunk at a time against us token by token, decays a head / a key channel / no delta with 64
+# heads of 64): one row of 64 tokens 26/36/29 against 24/23/26, of 128 29/40/36 against 45/43/49, of 2,048 186/245/231 against 685/648/738; 16 rows of
+# 32 tokens 90/120/141 against 86/104/145, of 64 92/125/157 against 166/200/282.  The line is drawn on what a captured step takes from the host, tokens and rows.
+CHUNKED_MIN_TOKENS = 128
+CHUNKED_MIN_TOKENS_A_ROW = 64
+CHUNKED_SCRATCH_FLOATS = 64 * 1024 * 1024  # what the chunks' products may take between the two kernels; more heads than fit go one group behind the other
+
+
+def chunked_recurrence_ok(tokens: int, rows: int, dim: int, vdim: int) -> bool:
+    """Whether a step's recurrences run a chunk of tokens at a time (``chunked_recurrence``) rather than token by token: rows of
+    whole 16 bytes, a state of up to 128 key channels, and enough tokens a row that a row's chunks beat its walk."""
+    return dim % 4 == 0 and 4 <= dim <= 128 and vdim % 4 == 0 and tokens >= CHUNKED_MIN_TOKENS and tokens >= CHUNKED_MIN_TOKENS_A_ROW * rows
+
+
+def chunked_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, states: torch.Tensor,
+                       out: torch.Tensor, *, qo_indptr: torch.Tensor, state_slots: torch.Tensor, kv_heads: int, dim: int, heads: int, vdim: int,
+                       workspace, delta: bool = True, channel_decay: bool = False, flag: Optional[torch.Tensor] = None) -> None:
+    """What ``delta_recurrence`` computes (``delta=False``: what ``ssm_recurrence`` computes, with q = c, k = b, v = x, beta = dt), a chunk of
+    64 tokens at a time as products in 32-bit.  The sums' order follows the chunks, so a row's bits depend on where its
+    portions were cut; the 32-bit mode, which promises otherwise, walks token by token."""
+    what = "chunked_recurrence"
+    _need_cuda(what, q, k, v, beta, decay, states, out, qo_indptr, state_slots, flag)
+    _need_i32(what, qo_indptr, state_slots)
+    for tensor in (q, k, v, beta, decay, states, out):
+        if tensor.dtype != torch.float32 or not tensor.is_contiguous():
+            raise KernelError(f"{what}: contiguous fp32 tensors only")
+    T, rows = q.shape[0], qo_indptr.numel() - 1
+    if tuple(states.shape[1:]) != (heads, vdim, dim) or out.numel() != v.numel() or v.numel() != T * heads * vdim:
+        raise KernelError(f"{what}: the state must be [slots, heads, vdim, dim] and the output as large as v")
+    if q.numel() != T * kv_heads * dim or k.numel() != q.numel() or beta.numel() != T * heads or decay.numel() != T * heads * (dim if channel_decay else 1):
+        raise KernelError(f"{what}: the keys, queries, betas or decays do not fit the sizes")
+    if channel_decay and not delta:
+        raise KernelError(f"{what}: a decay a key channel comes with the delta")
+    size_of = _fn("chunked_recurrence", "kb_chunked_recurrence_scratch", [c_int] * 6)
+    chunks = min(T, T // CHUNKED_TOKENS + rows)  # every row's last chunk may be a short one
+    sharing = heads // kv_heads
+    unit = chunks * size_of(dim, vdim, int(delta), int(channel_decay), sharing, sharing)
+    group = sharing * min(kv_heads, max(1, CHUNKED_SCRATCH_FLOATS // unit))
+    scratch = workspace.flat("recurrence.chunks", group // sharing * unit, torch.float32)
+    fn = _fn("chunked_recurrence", "kb_chunked_recurrence",
+             [c_void_p] * 8 + [c_int] * 4 + [c_void_p] + [c_int] * 5 + [c_void_p, ctypes.c_longlong, c_void_p, c_void_p])
+    _check(fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(), states.data_ptr(), qo_indptr.data_ptr(), state_slots.data_ptr(),
+              kv_heads, dim, heads, vdim, out.data_ptr(), rows, chunks, int(delta), int(channel_decay), group, scratch.data_ptr(), scratch.numel(), _ptr(flag), _stream()),
+           what, launches=2 * -(-heads // group))
+
+
 def delta_gated_norm(o: torch.Tensor, packed: torch.Tensor, gate_offset: int, weight: torch.Tensor, eps: float, out: torch.Tensor, *,
                      heads: int, vdim: int, gate_activation: str = "silu") -> None:
     """out[t, h] = o[t, h] / rms(o[t, h]) * weight * act(gate[t, h]); the gate is columns

@@ -50,6 +50,7 @@ LIBRARIES: dict[str, list[str]] = {
     "layernorm": [],
     "projection_rope": [],
     "delta_rule": [],
+    "chunked_recurrence": [],
     "ssm": [],
     "rglru": [],
     "rglru_tc5": [],

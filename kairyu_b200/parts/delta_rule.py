@@ -167,8 +167,12 @@ class GatedDeltaRule(Mixer):
             a_log=self.a_log, dt_bias=self.dt_bias, q=q, k=k, v=v, beta=beta, decay=decay, flag=ctx.error_flag, channel_a=channel_a, **sizes,
         )
         read_out = ws.buffer("delta.o", tokens, self.v_size, f32)
-        kernels.delta_recurrence(q, k, v, beta, decay, memory, read_out, qo_indptr=ctx.qo_indptr, state_slots=ctx.state_slots,
-                                 channel_decay=self.channel_decay, **sizes)
+        where = dict(qo_indptr=ctx.qo_indptr, state_slots=ctx.state_slots, channel_decay=self.channel_decay, **sizes)
+        # the 32-bit mode walks token by token: its results do not depend on where a prompt was cut
+        if self.dtype != torch.float32 and x.is_cuda and kernels.chunked_recurrence_ok(tokens, ctx.num_rows, self.head_dim, self.value_dim):
+            kernels.chunked_recurrence(q, k, v, beta, decay, memory, read_out, workspace=ws, flag=ctx.error_flag, **where)
+        else:
+            kernels.delta_recurrence(q, k, v, beta, decay, memory, read_out, **where)
         normed = ws.buffer("delta.normed", tokens, self.v_size, self.dtype)
         if self.gate_rank:
             gate = ws.buffer("delta.gate", tokens, self.v_size, self.dtype)

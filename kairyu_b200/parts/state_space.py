@@ -135,7 +135,12 @@ class StateSpaceDual(Mixer):
             state_slots=ctx.state_slots, a_log=self.a_log, dt_bias=self.dt_bias, x=xs, b=b, c=c, dt=dt, decay=decay, flag=ctx.error_flag, **sizes,
         )
         read_out = ws.buffer("ssm.y", tokens, self.inner, f32)
-        kernels.ssm_recurrence(c, b, xs, dt, decay, memory, read_out, qo_indptr=ctx.qo_indptr, state_slots=ctx.state_slots, **sizes)
+        # the 32-bit mode walks token by token: its results do not depend on where a prompt was cut
+        if self.dtype != torch.float32 and x.is_cuda and kernels.chunked_recurrence_ok(tokens, ctx.num_rows, self.state_size, self.value_dim):
+            kernels.chunked_recurrence(c, b, xs, dt, decay, memory, read_out, qo_indptr=ctx.qo_indptr, state_slots=ctx.state_slots, kv_heads=self.groups,
+                                       dim=self.state_size, heads=self.num_heads, vdim=self.value_dim, delta=False, workspace=ws, flag=ctx.error_flag)
+        else:
+            kernels.ssm_recurrence(c, b, xs, dt, decay, memory, read_out, qo_indptr=ctx.qo_indptr, state_slots=ctx.state_slots, **sizes)
         normed = ws.buffer("ssm.normed", tokens, self.inner, self.dtype)
         kernels.ssm_gated_norm(read_out, xs, self.skip, packed[:, : self.inner], self.out_norm, self.norm_eps, normed,
                                heads=self.num_heads, vdim=self.value_dim, norm_groups=self.norm_groups)
