@@ -480,6 +480,7 @@ def paged_attention_generic(
     sinks: Optional[torch.Tensor] = None,
     value_dim: Optional[int] = None,
     out_head_stride: Optional[int] = None,
+    workspace=None,
 ) -> None:
     """fp32-arithmetic attention of every token in ``q`` over its request's pages.
 
@@ -489,6 +490,7 @@ def paged_attention_generic(
     leading columns of a value row are used; with ``v_cache`` the key cache itself, a row's first
     ``value_dim`` columns are its value.  ``out_head_stride`` (default: value_dim): where head h's
     output starts in its token's row, h * out_head_stride (the columns behind value_dim stay as they are).
+    ``workspace``: a step of single tokens takes scratch from it to spread long rows' keys over the device (the results are the same without).
     """
     _need_cuda("paged_attention_generic", q, out, k_cache, v_cache, positions, row_ids, block_table, flag, sinks)
     if sinks is not None and (sinks.dtype != torch.float32 or sinks.numel() != num_q_heads or not sinks.is_contiguous()):
@@ -507,17 +509,28 @@ def paged_attention_generic(
     fn = _fn(
         "attention_generic",
         "kb_paged_attention_generic",
-        [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p],
+        [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_int, c_int, c_void_p,
+         ctypes.c_longlong, c_void_p, c_void_p],
     )
     value_dim = int(head_dim if value_dim is None else value_dim)
+    rows = block_table.shape[0]
+    scratch = None
+    if workspace is not None and T == rows and q.dtype == torch.float32:
+        need_fn = _fn("attention_generic", "kb_paged_attention_generic_scratch", [c_int] * 6)
+        need_fn.restype = ctypes.c_longlong
+        need = need_fn(T, num_q_heads, num_kv_heads, head_dim, value_dim, block_table.shape[1] * page_size)
+        if need:
+            scratch = workspace.flat("attn.generic_parts", need, torch.float32)
     _check(
         fn(
             q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
             _is_bf16(q, "paged_attention_generic"), positions.data_ptr(), row_ids.data_ptr(), block_table.data_ptr(),
             block_table.shape[1], T, num_q_heads, num_kv_heads, head_dim, page_size, num_pages, float(scale),
-            int(window), _ptr(sinks), value_dim, int(value_dim if out_head_stride is None else out_head_stride), _ptr(flag), _stream(),
+            int(window), _ptr(sinks), value_dim, int(value_dim if out_head_stride is None else out_head_stride),
+            rows, _ptr(scratch), 0 if scratch is None else scratch.numel(), _ptr(flag), _stream(),
         ),
         "paged_attention_generic",
+        launches=1 if scratch is None else 2,
     )
 
 

@@ -104,6 +104,7 @@ def run_paged_attention(
             sinks=sinks,
             value_dim=value_dim,
             out_head_stride=head_dim,
+            **({"workspace": ctx.workspace} if qkv.is_cuda else {}),
         )
         return
     num_tiles, tile_rows, tile_starts = ctx.tiles[kernels.attention_prefill_tile_rows(head_dim)]
