@@ -146,6 +146,13 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool live) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
+// two multiply-adds in one instruction, each rounded as fmaf rounds
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
 // (m, l, acc) of the segments so far with one more: the same few operations wherever segments are merged
 struct Merge {
     float before, after;  // factors of the sums so far and of the segment's
@@ -265,18 +272,19 @@ paged_attention_tiled_kernel(const Tiled p) {
         if (more) look_up(tile + 1);
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        // scores: a thread's keys are tx, tx + 16, tx + 32, tx + 48; 32 channels at a time into one sum, those sums into another
+        // scores: a thread's keys are tx, tx + 16, tx + 32, tx + 48; 32 channels at a time, the even and the odd ones
+        // into a sum each, those sums into another
         float s[TM][4];
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
         for (int d0 = 0; d0 < DP; d0 += 32) {
-            float part[TM][4];
+            float2 part[TM][4];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
+                for (int j = 0; j < 4; ++j) part[i][j] = make_float2(0.0f, 0.0f);
 #pragma unroll
             for (int d = 0; d < 32; d += 4) {
                 float4 kv[4];
@@ -287,17 +295,15 @@ paged_attention_tiled_kernel(const Tiled p) {
                     const float4 qv = *reinterpret_cast<const float4*>(qs + (ty * TM + i) * LD + d0 + d);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        part[i][j] = fmaf(qv.x, kv[j].x, part[i][j]);
-                        part[i][j] = fmaf(qv.y, kv[j].y, part[i][j]);
-                        part[i][j] = fmaf(qv.z, kv[j].z, part[i][j]);
-                        part[i][j] = fmaf(qv.w, kv[j].w, part[i][j]);
+                        part[i][j] = fma2(make_float2(qv.x, qv.y), make_float2(kv[j].x, kv[j].y), part[i][j]);
+                        part[i][j] = fma2(make_float2(qv.z, qv.w), make_float2(kv[j].z, kv[j].w), part[i][j]);
                     }
                 }
             }
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] += part[i][j];
+                for (int j = 0; j < 4; ++j) s[i][j] += part[i][j].x + part[i][j].y;
         }
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
@@ -343,10 +349,10 @@ paged_attention_tiled_kernel(const Tiled p) {
 #pragma unroll
                     for (int i = 0; i < TM; ++i) {
                         const float w = j == 0 ? e[i].x : j == 1 ? e[i].y : j == 2 ? e[i].z : e[i].w;
-                        acc[i][4 * c] = fmaf(w, v.x, acc[i][4 * c]);
-                        acc[i][4 * c + 1] = fmaf(w, v.y, acc[i][4 * c + 1]);
-                        acc[i][4 * c + 2] = fmaf(w, v.z, acc[i][4 * c + 2]);
-                        acc[i][4 * c + 3] = fmaf(w, v.w, acc[i][4 * c + 3]);
+                        const float2 ww = make_float2(w, w);
+                        const float2 lo = fma2(ww, make_float2(v.x, v.y), make_float2(acc[i][4 * c], acc[i][4 * c + 1]));
+                        const float2 hi = fma2(ww, make_float2(v.z, v.w), make_float2(acc[i][4 * c + 2], acc[i][4 * c + 3]));
+                        acc[i][4 * c] = lo.x, acc[i][4 * c + 1] = lo.y, acc[i][4 * c + 2] = hi.x, acc[i][4 * c + 3] = hi.y;
                     }
                 }
             }

@@ -5,12 +5,23 @@
 // additions, not of 8,192), so a row's result does not depend on M, on the tile's shape or on which tile
 // it falls in: the 32-bit path is bit-stable however a prompt is cut into steps.
 //
-// What bounds it: the FMA pipes, 128 a cycle and SM, for which every thread keeps a TM x TN block of outputs in registers, so that
-// the factors' reads from shared memory (TM + TN floats a k) stay below the multiply-adds (TM * TN); the next BK columns of both factors are
+// What bounds it: shared memory hands out 128 bytes a cycle and SM, one float for every four of the 128 multiply-adds, so a thread's block of
+// TM x TN outputs takes (TM + TN) floats a k where TM * TN / 4 are free: 8 x 8 outputs are level, 16 x 8 are ahead.  Two multiply-adds go in one
+// instruction, which leaves issue slots for those reads (700 x 3,072 x 2,048: 485 -> 217 us, 41 TFLOP/s; with 4 x 4 outputs a thread and
+// loads that waited for the products 466; 2,048 x 8,192 x 2,048: 1,278 us, 54 TFLOP/s, and 3,090).
+// 16 x 8 outputs leave no registers for the second accumulators, which are needed
+// once in 256 terms and stand in shared memory (SPILL).  The next BK columns of both factors are
 // fetched into registers while this BK is multiplied and go into the other half of shared memory.
 #include "common.cuh"
 
 #define F32_SUM_BLOCK 256  // terms a first-level accumulator takes before it is added to the second
+
+// Two multiply-adds in one instruction (each rounded as fmaf rounds), with one factor for both
+__device__ __forceinline__ void fma_pair(float& x0, float& x1, float a0, float a1, float b) {
+    asm("{\n .reg .b64 x, a, b;\n mov.b64 x, {%0, %1};\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n fma.rn.f32x2 x, a, b, x;\n mov.b64 {%0, %1}, x;\n}\n"
+        : "+f"(x0), "+f"(x1)
+        : "f"(a0), "f"(a1), "f"(b));
+}
 
 // Four consecutive floats of row r at column k, zeros outside the matrix; `wide`: rows are whole aligned 16-byte groups
 __device__ __forceinline__ float4 f32_fetch(const float* __restrict__ a, int ld, int r, int rows, int k, int K, bool wide) {
@@ -21,7 +32,7 @@ __device__ __forceinline__ float4 f32_fetch(const float* __restrict__ a, int ld,
 }
 
 // A thread's TM rows are groups of G that lie BM / (TM / G) apart (so that a warp's 16-byte reads of one group are side by side), its TN columns likewise.
-template <int BM, int BN, int TM, int TN, int BK>
+template <int BM, int BN, int TM, int TN, int BK, bool SPILL>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int ldw,
                 const float* __restrict__ bias, float* __restrict__ y, int ldy, int M, int N, int K, int x_wide, int w_wide) {
@@ -30,17 +41,23 @@ gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
     constexpr int LA = BM + 4, LB = BN + 4;
     constexpr int NA = BM * BK / 4 / THREADS, NB = BN * BK / 4 / THREADS;
     static_assert(NA * 4 * THREADS == BM * BK && NB * 4 * THREADS == BN * BK && F32_SUM_BLOCK % BK == 0, "whole loads");
-    __shared__ __align__(16) float As[2][BK][LA];
-    __shared__ __align__(16) float Bs[2][BK][LB];
+    extern __shared__ __align__(16) float sm[];
+    float(*As)[BK][LA] = reinterpret_cast<float(*)[BK][LA]>(sm);
+    float(*Bs)[BK][LB] = reinterpret_cast<float(*)[BK][LB]>(sm + 2 * BK * LA);
+    float* totals = sm + 2 * BK * (LA + LB) + threadIdx.x;  // SPILL: TM * TN of them, THREADS apart
     const int tid = threadIdx.x, tx = tid % COLS, ty = tid / COLS;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     pdl_wait();
 
-    float acc[TM][TN], total[TM][TN];
+    float acc[TN][TM], total[SPILL ? 1 : TM][SPILL ? 1 : TN];
+    auto second = [&](int i, int j) -> float& {
+        if constexpr (SPILL) return totals[(i * TN + j) * THREADS];
+        else return total[i][j];
+    };
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = total[i][j] = 0.0f;
+        for (int j = 0; j < TN; ++j) acc[j][i] = second(i, j) = 0.0f;
     float4 na[NA], nb[NB];
     auto fetch = [&](int k0) {
 #pragma unroll
@@ -79,8 +96,8 @@ gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    total[i][j] += acc[i][j];
-                    acc[i][j] = 0.0f;
+                    second(i, j) += acc[j][i];
+                    acc[j][i] = 0.0f;
                 }
         }
         const bool more = k0 + BK < K;
@@ -111,9 +128,9 @@ gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
                 }
             }
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int j = 0; j < TN; ++j)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int i = 0; i < TM; i += 2) fma_pair(acc[j][i], acc[j][i + 1], a[i], a[i + 1], b[j]);
         }
         if (more) place(buf ^ 1);  // the other half was read before the last barrier
         __syncthreads();
@@ -126,19 +143,22 @@ gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
         for (int j = 0; j < TN; ++j) {
             const int n = n0 + col_at(j);
             if (n >= N) continue;
-            float v = total[i][j] + acc[i][j];
+            float v = second(i, j) + acc[j][i];
             if (bias) v += bias[n];
             y[(size_t)m * ldy + n] = v;
         }
     }
 }
 
-template <int BM, int BN, int TM, int TN, int BK>
+template <int BM, int BN, int TM, int TN, int BK, bool SPILL>
 static int launch_gemm_f32(const float* x, int ldx, const float* w, int ldw, const float* bias, float* y, int ldy, int M, int N, int K, cudaStream_t stream) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return KB_ERR_UNSUPPORTED_SIZE;
     const int x_wide = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0, w_wide = K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)w & 15) == 0;
-    kb_launch(gemm_f32_kernel<BM, BN, TM, TN, BK>, grid, dim3((BM / TM) * (BN / TN)), 0, stream, x, ldx, w, ldw, bias, y, ldy, M, N, K, x_wide, w_wide);
+    constexpr size_t bytes = (2 * BK * (BM + BN + 8) + (SPILL ? BM * BN : 0)) * sizeof(float);
+    if (bytes > 48 * 1024)
+        if (cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TM, TN, BK, SPILL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) return (int)e;
+    kb_launch(gemm_f32_kernel<BM, BN, TM, TN, BK, SPILL>, grid, dim3((BM / TM) * (BN / TN)), bytes, stream, x, ldx, w, ldw, bias, y, ldy, M, N, K, x_wide, w_wide);
     return kb_launch_result();
 }
 
@@ -149,19 +169,20 @@ KB_EXPORT int kb_gemm_f32(const float* x, int ldx, const float* w, int ldw, cons
     if (K < 1) return KB_ERR_BAD_ARG;
     if (M > 65535 * 64) return KB_ERR_UNSUPPORTED_SIZE;
 #define F32_ARGS x, ldx, w, ldw, bias, y, ldy, M, N, K, stream
-    // A few rows: what counts is that many blocks stream the weight.
-    if (M <= 16) return launch_gemm_f32<16, 32, 2, 2, 64>(F32_ARGS);
+    // A few rows: what counts is that many blocks stream the weight (N = 3,072, K = 2,048: 37 us at 16 rows, where tiles of 64 x 64 take 91).
+    if (M <= 96) return launch_gemm_f32<16, 32, 2, 2, 64, false>(F32_ARGS);
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 148;
-    // The larger a tile, the fewer reads a multiply-add; the smaller, the less of the last wave is empty.  Time in units of outputs an SM
-    // multiplies one behind the other, a tile's rate as measured relative to the largest.
-    auto waves = [&](int bm, int bn, int resident, double rate) {
+    // The larger a tile, the fewer reads a multiply-add; the smaller, the more evenly the outputs lie on the SMs (tiles on one SM share its pipes).  Time in
+    // outputs of the fullest SM, over a tile's rate relative to the largest.
+    auto time = [&](int bm, int bn, double rate) {
         const long long blocks = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-        return (double)((blocks + (long long)sms * resident - 1) / ((long long)sms * resident)) * resident * bm * bn / rate;
+        return (double)((blocks + sms - 1) / sms) * bm * bn / rate;
     };
-    const double large = waves(128, 128, 1, 1.0), middle = waves(64, 128, 2, 0.9), small = waves(64, 64, 3, 0.7);
-    if (large <= middle && large <= small) return launch_gemm_f32<128, 128, 8, 8, 16>(F32_ARGS);
-    if (middle <= small) return launch_gemm_f32<64, 128, 8, 4, 16>(F32_ARGS);
-    return launch_gemm_f32<64, 64, 4, 4, 16>(F32_ARGS);
+    const double huge = time(128, 128, 1.0), large = time(96, 128, 0.95), middle = time(64, 128, 0.8), small = time(64, 64, 0.5);
+    if (huge <= large && huge <= middle && huge <= small) return launch_gemm_f32<128, 128, 16, 8, 16, true>(F32_ARGS);
+    if (large <= middle && large <= small) return launch_gemm_f32<96, 128, 12, 8, 16, true>(F32_ARGS);
+    if (middle <= small) return launch_gemm_f32<64, 128, 8, 8, 16, true>(F32_ARGS);
+    return launch_gemm_f32<64, 64, 4, 4, 16, false>(F32_ARGS);
 #undef F32_ARGS
 }
