@@ -129,6 +129,59 @@ delta_prepare_kernel(const TA* __restrict__ proj, int stride, const float* __res
     }
 }
 
+// The same for heads of up to 128 channels in whole groups of four: a warp a head (or 128 channels of v), four channels a lane, over a few neighbouring tokens.
+// What bounds it is instructions (the exponentials of silu, the decays); what is saved is the look-ups a token and channel and two thirds
+// of the reads (5,001 tokens of 32 heads with a decay a key channel: 341 us before).
+template <typename TA, int NT>
+__global__ void __launch_bounds__(128)
+delta_prepare_wide_kernel(const TA* __restrict__ proj, int stride, const float* __restrict__ gates, int gate_stride, const float* __restrict__ channel_a,
+                          const float* __restrict__ taps, const float* __restrict__ conv_state, const int* __restrict__ row_ids, const int* __restrict__ qo_indptr,
+                          const int* __restrict__ state_slots, const float* __restrict__ A_log, const float* __restrict__ dt_bias, int KH, int D, int H, int V,
+                          float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vv, float* __restrict__ beta, float* __restrict__ decay, int num_rows, int T,
+                          int tokens, int* flag) {
+    const int t0 = blockIdx.x * tokens, end = min(T, t0 + tokens);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int C = 2 * KH * D + H * V;
+    const int unit = blockIdx.y * 4 + warp;
+    pdl_wait();
+    if (blockIdx.y == 0 && threadIdx.x < 32 && flag)
+        for (int t = t0 + lane; t < end; t += 32)
+            if (row_ids[t] < 0 || row_ids[t] >= num_rows) atomicOr(flag, KB_FLAG_BAD_ROW);
+    if (unit < 2 * KH) {
+        const int c = min(4 * lane, D - 4);  // lanes behind the head's last group repeat it and count for nothing
+        const bool live = 4 * lane < D;
+        float* dst = unit < KH ? qn + (size_t)unit * D : kn + (size_t)(unit - KH) * D;
+        const float times = unit < KH ? rsqrtf((float)D) : 1.0f;
+        convolve_four<TA, NT, false>(proj, stride, conv_state, taps, nullptr, C, unit * D + c, row_ids, qo_indptr, state_slots, num_rows, t0, tokens, T, [&](int t, float4 z) {
+            z = silu_four(z);
+            const float ss = warp_sum(live ? (z.x * z.x + z.y * z.y) + (z.z * z.z + z.w * z.w) : 0.0f);
+            const float scale = rsqrtf(ss + 1e-6f) * times;
+            if (live) store_four<float>(dst + (size_t)t * KH * D + c, make_float4(z.x * scale, z.y * scale, z.z * scale, z.w * scale));
+        });
+    } else {
+        const int c = (unit - 2 * KH) * 128 + 4 * lane;
+        if (c < H * V)
+            convolve_four<TA, NT, false>(proj, stride, conv_state, taps, nullptr, C, 2 * KH * D + c, row_ids, qo_indptr, state_slots, num_rows, t0, tokens, T,
+                                         [&](int t, float4 z) { store_four<float>(vv + (size_t)t * H * V + c, silu_four(z)); });
+    }
+    auto decay_of = [](float rate, float a) { return expf(-rate * softplus_f(a)); };
+    if (blockIdx.y == 0)
+        for (int i = threadIdx.x; i < (end - t0) * H; i += blockDim.x) {
+            const int t = t0 + i / H, h = i % H;
+            beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-gates[(size_t)t * gate_stride + h]));
+            if (!channel_a) decay[(size_t)t * H + h] = decay_of(expf(A_log[h]), gates[(size_t)t * gate_stride + H + h] + dt_bias[h]);
+        }
+    if (channel_a)
+        for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * 4; i < H * D; i += gridDim.y * blockDim.x * 4) {
+            const float rate = expf(A_log[i / D]);
+            const float4 b = load_four<float>(dt_bias + i);
+            for (int t = t0; t < end; ++t) {
+                const float4 a = load_four<float>(channel_a + (size_t)t * H * D + i);
+                store_four<float>(decay + (size_t)t * H * D + i, make_float4(decay_of(rate, a.x + b.x), decay_of(rate, a.y + b.y), decay_of(rate, a.z + b.z), decay_of(rate, a.w + b.w)));
+            }
+        }
+}
+
 // gate: [tokens, H * V] columns of a row of `gate_stride` entries; sigmoid_gate: sigmoid(gate), else silu(gate)
 template <typename TA>
 __global__ void __launch_bounds__(128)
@@ -152,6 +205,27 @@ delta_gated_norm_kernel(const float* __restrict__ o, const TA* __restrict__ gate
     }
 }
 
+// The same for heads of up to 128 columns in whole groups of four: a warp a (token, head), four columns a lane, read once.
+template <typename TA>
+__global__ void __launch_bounds__(256)
+delta_gated_norm_wide_kernel(const float* __restrict__ o, const TA* __restrict__ gate, int gate_stride, int sigmoid_gate, const float* __restrict__ w, float eps,
+                             int H, int V, TA* __restrict__ out, int T) {
+    const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // (token, head)
+    const int e = 4 * (threadIdx.x & 31);
+    pdl_wait();
+    if (unit >= (long long)T * H) return;
+    const int t = (int)(unit / H), h = (int)(unit % H);
+    const bool live = e < V;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 x = live ? load_four<float>(o + unit * V + e) : none;
+    const float4 z = live ? load_four<TA>(gate + (size_t)t * gate_stride + h * V + e) : none;
+    const float4 weight = live ? load_four<float>(w + e) : none;
+    const float ss = warp_sum((x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w));
+    const float inv = rsqrtf(ss / (float)V + eps);
+    auto gated = [&](float v, float weight, float z) { return v * inv * weight * (sigmoid_gate ? 1.0f / (1.0f + expf(-z)) : silu_f(z)); };
+    if (live) store_four<TA>(out + unit * V + e, make_float4(gated(x.x, weight.x, z.x), gated(x.y, weight.y, z.y), gated(x.z, weight.z, z.z), gated(x.w, weight.w, z.w)));
+}
+
 // channel_a null: `gates` is [tokens, 2H] (beta's logits, then a) and the decay one number a head ([tokens, H]);
 // else `gates` is [tokens, H], channel_a [tokens, H * D], dt_bias [H * D] and the decay [tokens, H, D].
 KB_EXPORT int kb_delta_prepare(const void* proj, int stride, int is_bf16, const float* gates, const float* channel_a, const float* taps, int n,
@@ -168,13 +242,24 @@ KB_EXPORT int kb_delta_prepare(const void* proj, int stride, int is_bf16, const 
 #define LAUNCH(TA, NT)                                                                                                        \
     kb_launch(delta_prepare_kernel<TA, NT>, dim3(T, (2 * KH + H + 3) / 4), dim3(128), 0, stream, (const TA*)proj, stride, gates, gate_stride, channel_a, taps, n, \
               (const float*)conv_state, row_ids, qo_indptr, state_slots, A_log, dt_bias, KH, D, H, V, qn, kn, vv, beta, decay, num_rows, flag)
+    const int units = 2 * KH + (H * V + 127) / 128;
+    const int tokens = convolve_tokens(T, (units + 3) / 4);
+    // by widths and alignment alone, so that a token's bits do not depend on the step
+    const bool wide = n <= 4 && D % 4 == 0 && D <= 128 && V % 4 == 0 && stride % 4 == 0 && aligned16(proj) && aligned16(taps) && (n == 1 || aligned16(conv_state)) && aligned16(qn)
+        && aligned16(kn) && aligned16(vv) && (!channel_a || (aligned16(channel_a) && aligned16(dt_bias) && aligned16(decay)));
+#define LAUNCH_WIDE(TA, NT)                                                                                                   \
+    kb_launch(delta_prepare_wide_kernel<TA, NT>, dim3((T + tokens - 1) / tokens, (units + 3) / 4), dim3(128), 0, stream, (const TA*)proj, stride, gates, gate_stride, \
+              channel_a, taps, (const float*)conv_state, row_ids, qo_indptr, state_slots, A_log, dt_bias, KH, D, H, V, qn, kn, vv, beta, decay, num_rows, T, tokens, flag)
 #define PICK(TA)                                                                                                              \
     do {                                                                                                                      \
-        if (n == 1) LAUNCH(TA, 1); else if (n == 2) LAUNCH(TA, 2); else if (n == 3) LAUNCH(TA, 3); else if (n == 4) LAUNCH(TA, 4); \
+        if (wide) {                                                                                                           \
+            if (n == 1) LAUNCH_WIDE(TA, 1); else if (n == 2) LAUNCH_WIDE(TA, 2); else if (n == 3) LAUNCH_WIDE(TA, 3); else LAUNCH_WIDE(TA, 4); \
+        } else if (n == 1) LAUNCH(TA, 1); else if (n == 2) LAUNCH(TA, 2); else if (n == 3) LAUNCH(TA, 3); else if (n == 4) LAUNCH(TA, 4); \
         else LAUNCH(TA, 0);                                                                                                   \
     } while (0)
     if (is_bf16) PICK(__nv_bfloat16); else PICK(float);
 #undef PICK
+#undef LAUNCH_WIDE
 #undef LAUNCH
     int code = kb_launch_result();
     if (code != 0 || n == 1) return code;
@@ -195,6 +280,14 @@ KB_EXPORT int kb_delta_gated_norm(const float* o, const void* gate, int gate_str
     if (T == 0) return 0;
     if (!o || !gate || !w || !out) return KB_ERR_NULL;
     if (H < 1 || H > 4 * 65535) return KB_ERR_UNSUPPORTED_SIZE;
+    if (V % 4 == 0 && V <= 128 && gate_stride % 4 == 0 && aligned16(o) && aligned16(w) && ((uintptr_t)gate & (is_bf16 ? 7 : 15)) == 0 && aligned16(out)) {
+        const unsigned blocks = (unsigned)(((long long)T * H + 7) / 8);
+        if (is_bf16)
+            kb_launch(delta_gated_norm_wide_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, o, (const __nv_bfloat16*)gate, gate_stride, sigmoid_gate, w, eps, H, V, (__nv_bfloat16*)out, T);
+        else
+            kb_launch(delta_gated_norm_wide_kernel<float>, dim3(blocks), dim3(256), 0, stream, o, (const float*)gate, gate_stride, sigmoid_gate, w, eps, H, V, (float*)out, T);
+        return kb_launch_result();
+    }
     if (is_bf16)
         kb_launch(delta_gated_norm_kernel<__nv_bfloat16>, dim3(T, (H + 3) / 4), dim3(128), 0, stream, o, (const __nv_bfloat16*)gate, gate_stride, sigmoid_gate, w, eps, H, V, (__nv_bfloat16*)out);
     else

@@ -37,6 +37,89 @@ __device__ __forceinline__ float conv_input(const TA* __restrict__ proj, int str
     return kept[(size_t)((n - 1) + (o - back)) * C + c];
 }
 
+// four neighbouring columns in 32-bit
+template <typename TA>
+__device__ __forceinline__ float4 load_four(const TA* at);
+template <>
+__device__ __forceinline__ float4 load_four<float>(const float* at) { return *reinterpret_cast<const float4*>(at); }
+template <>
+__device__ __forceinline__ float4 load_four<__nv_bfloat16>(const __nv_bfloat16* at) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(at);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename TA>
+__device__ __forceinline__ void store_four(TA* at, float4 v);
+template <>
+__device__ __forceinline__ void store_four<float>(float* at, float4 v) { *reinterpret_cast<float4*>(at) = v; }
+template <>
+__device__ __forceinline__ void store_four<__nv_bfloat16>(__nv_bfloat16* at, float4 v) {
+    __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(at) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+
+// A short causal convolution of four neighbouring channels over `tokens` neighbouring tokens from t0 on: a thread keeps the inputs that the next token
+// needs, so that an input is read once.  `use(t, z)` takes each token's four sums; a token whose row is out of range is passed over with use never
+// called.  OLDEST_FIRST: the order in which the taps are added (with `bias` before them).  Channels are c .. c + 3 of C; rows of proj, kept inputs and taps
+// are whole aligned groups of four.
+template <typename TA, int NT, bool OLDEST_FIRST, typename Use>
+__device__ __forceinline__ void convolve_four(const TA* __restrict__ proj, int stride, const float* __restrict__ conv_state, const float* __restrict__ taps,
+                                              const float* __restrict__ bias, int C, int c, const int* __restrict__ row_ids, const int* __restrict__ qo_indptr,
+                                              const int* __restrict__ state_slots, int num_rows, int t0, int tokens, int T, Use use) {
+    float w[4][NT];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) w[e][j] = taps[(size_t)(c + e) * NT + j];
+    const float4 start = bias ? load_four<float>(bias + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 past[NT > 1 ? NT - 1 : 1];  // [0]: the newest
+    int held = -1;                     // the row they are of
+    const int end = min(T, t0 + tokens);
+    float4 next = load_four<TA>(proj + (size_t)t0 * stride + c);
+    for (int t = t0; t < end; ++t) {
+        const float4 x = next;
+        if (t + 1 < end) next = load_four<TA>(proj + (size_t)(t + 1) * stride + c);
+        const int row = row_ids[t];
+        if (row < 0 || row >= num_rows) {
+            held = -1;
+            continue;
+        }
+        if (NT > 1 && row != held) {
+            const int o = t - qo_indptr[row];
+            const float* kept = conv_state + (size_t)state_slots[row] * (NT - 1) * C + c;
+#pragma unroll
+            for (int back = 1; back < NT; ++back)
+                past[back - 1] = o - back >= 0 ? load_four<TA>(proj + (size_t)(t - back) * stride + c) : load_four<float>(kept + (size_t)((NT - 1) + (o - back)) * C);
+            held = row;
+        }
+        float4 z = start;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const int back = OLDEST_FIRST ? NT - 1 - i : i;
+            const float4 v = back == 0 ? x : past[back > 0 ? back - 1 : 0];
+            z.x = fmaf(w[0][NT - 1 - back], v.x, z.x);
+            z.y = fmaf(w[1][NT - 1 - back], v.y, z.y);
+            z.z = fmaf(w[2][NT - 1 - back], v.z, z.z);
+            z.w = fmaf(w[3][NT - 1 - back], v.w, z.w);
+        }
+        if constexpr (NT > 1) {
+#pragma unroll
+            for (int i = NT - 2; i > 0; --i) past[i] = past[i - 1];
+            past[0] = x;
+        }
+        use(t, z);
+    }
+}
+__device__ __forceinline__ float4 silu_four(float4 z) { return make_float4(silu_f(z.x), silu_f(z.y), silu_f(z.z), silu_f(z.w)); }
+
+// Tokens a thread convolves one behind the other: sixteen where that leaves blocks enough for the device (`across` blocks a token group), one in a short step.
+static inline int convolve_tokens(int T, int across) {
+    for (int tokens = 16; tokens > 1; tokens /= 4)
+        if ((long long)(T / tokens) * across >= 512) return tokens;
+    return 1;
+}
+static inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
 // per request: the last (n - 1) inputs of the step become the kept inputs; a thread reads all it needs of a
 // (request, channel) before it writes
 template <typename TA>

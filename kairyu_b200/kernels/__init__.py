@@ -2153,7 +2153,8 @@ def chunked_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: 
     chunks = min(T, T // CHUNKED_TOKENS + rows)  # every row's last chunk may be a short one
     sharing = heads // kv_heads
     unit = chunks * size_of(dim, vdim, int(delta), int(channel_decay), sharing, sharing)
-    group = sharing * min(kv_heads, max(1, CHUNKED_SCRATCH_FLOATS // unit))
+    groups = -(-kv_heads // min(kv_heads, max(1, CHUNKED_SCRATCH_FLOATS // unit)))
+    group = sharing * -(-kv_heads // groups)  # groups of one size
     scratch = workspace.flat("recurrence.chunks", group // sharing * unit, torch.float32)
     fn = _fn("chunked_recurrence", "kb_chunked_recurrence",
              [c_void_p] * 8 + [c_int] * 4 + [c_void_p] + [c_int] * 5 + [c_void_p, ctypes.c_longlong, c_void_p, c_void_p])
