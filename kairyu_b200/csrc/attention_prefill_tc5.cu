@@ -46,8 +46,10 @@
 //
 // Every wait on an mbarrier is bounded: a role that gives up raises KB_FLAG_TIMEOUT, lets the
 // other roles leave through a shared abort word, and the block frees its TMEM and returns.
-// Sizes: head_dim 64 or 128, page_size a power of two from 8 up; others go to the mma.sync
-// kernel of attention_mma.cuh.
+// Sizes: head_dim 64, 128 or 256, page_size a power of two from 8 up; others go to the mma.sync
+// kernel of attention_mma.cuh.  At 256 columns a block has the SM to itself and what bounds it is again the copies, 20 a key tile with pages of 16; the mma.sync
+// kernel's tiles of 64 queries read every key twice as often and their products run at a quarter of the rate (latent attention, 16 heads over one
+// row of 256 columns, 2,048 tokens in three portions behind up to 900: 335 -> 98 us).
 #include "softcap.cuh"
 #include "umma.cuh"
 
@@ -130,8 +132,8 @@ struct FaCfg {
     static constexpr size_t SMEM = OFF_BAR + NUM_BARS * 8 + 16;
     static constexpr int S_COL = 0;          // two S buffers of FA_BN columns each; P (bf16 pairs) overwrites the first half of its S
     static constexpr int O_COL = 2 * FA_BN;
-    static constexpr int TMEM_COLUMNS = 256;
-    static constexpr int BLOCKS_PER_SM = 2;
+    static constexpr int TMEM_COLUMNS = D > 128 ? 512 : 256;
+    static constexpr int BLOCKS_PER_SM = D > 128 ? 1 : 2;  // 256 columns: 193 KB of shared memory and 384 columns of tensor memory
 };
 
 template <int D, bool CAP>
@@ -1095,10 +1097,12 @@ __global__ void attention_prefill_tc5_merge_kernel(const float* __restrict__ par
         const float f = exp2f(m - big);
         den += part_ml[at * 2 + 1] * f;
         float part[PER];
-        if (PER == 4)
-            *reinterpret_cast<float4*>(part) = *reinterpret_cast<const float4*>(part_o + at * D + lane * PER);
-        else
+        if constexpr (PER >= 4) {
+#pragma unroll
+            for (int i = 0; i < PER; i += 4) *reinterpret_cast<float4*>(part + i) = *reinterpret_cast<const float4*>(part_o + at * D + lane * PER + i);
+        } else {
             *reinterpret_cast<float2*>(part) = *reinterpret_cast<const float2*>(part_o + at * D + lane * PER);
+        }
 #pragma unroll
         for (int i = 0; i < PER; ++i) acc[i] += part[i] * f;
     }
@@ -1116,10 +1120,9 @@ __global__ void attention_prefill_tc5_merge_kernel(const float* __restrict__ par
         __nv_bfloat162 two = __floats2bfloat162_rn(acc[i] * inv, acc[i + 1] * inv);
         packed[i / 2] = *reinterpret_cast<uint32_t*>(&two);
     }
-    if (PER == 4)
-        *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[PER / 2 - 1]);
-    else
-        *reinterpret_cast<uint32_t*>(dst) = packed[0];
+    if constexpr (PER == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    else if constexpr (PER == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
+    else *reinterpret_cast<uint32_t*>(dst) = packed[0];
 }
 
 static int fa_resident(int blocks_per_sm) {
@@ -1135,10 +1138,10 @@ static int fa_resident(int blocks_per_sm) {
 // long prompt: 4 tiles x 32 heads) would leave most of the device idle.  Every split gets at least
 // four key tiles of the longest row; at most eight splits.
 KB_EXPORT int kb_attention_prefill_tc5_splits(int D, int Hq, int num_tiles, int max_seq_len) {
-    if (D != 64 && D != 128) return 1;
+    if (D != 64 && D != 128 && D != 256) return 1;
     const long long blocks = (long long)Hq * num_tiles;
     if (blocks < 1) return 1;
-    const int resident = fa_resident(FaCfg<128>::BLOCKS_PER_SM);
+    const int resident = fa_resident(D == 256 ? FaCfg<256>::BLOCKS_PER_SM : FaCfg<128>::BLOCKS_PER_SM);
     long long splits = resident / blocks;
     const int key_tiles = (max_seq_len + FA_BN - 1) / FA_BN;
     if (splits > key_tiles / 4) splits = key_tiles / 4;
@@ -1206,7 +1209,7 @@ KB_EXPORT int kb_attention_prefill_tc5_two_tiles(int D, int Hq, int num_wide, in
 
 // 1 when (head_dim, page_size) fit this kernel.
 KB_EXPORT int kb_attention_prefill_tc5_supported(int D, int page_size) {
-    if (D != 64 && D != 128) return 0;
+    if (D != 64 && D != 128 && D != 256) return 0;
     if (page_size < 8 || (page_size & (page_size - 1)) != 0) return 0;
     return 1;
 }
@@ -1251,10 +1254,10 @@ KB_EXPORT int kb_attention_prefill_tc5(const void* map_q, const void* map_k, con
     const KbSoftcap cap = kb_softcap_of(softcap);
     if (cap.mode != KB_SOFTCAP_NONE) {
         if (two_tiles) return launch_two<true>(TWO_ARGS);
-        return D == 64 ? launch_fa<64, true>(ARGS) : launch_fa<128, true>(ARGS);
+        return D == 64 ? launch_fa<64, true>(ARGS) : D == 128 ? launch_fa<128, true>(ARGS) : launch_fa<256, true>(ARGS);
     }
     if (two_tiles) return launch_two<false>(TWO_ARGS);
-    return D == 64 ? launch_fa<64, false>(ARGS) : launch_fa<128, false>(ARGS);
+    return D == 64 ? launch_fa<64, false>(ARGS) : D == 128 ? launch_fa<128, false>(ARGS) : launch_fa<256, false>(ARGS);
 #undef TWO_ARGS
 #undef ARGS
 }

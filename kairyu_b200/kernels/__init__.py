@@ -908,10 +908,10 @@ def attention_prefill_tile_rows(head_dim: int) -> int:
 
 
 def attention_prefill_wide_tile_rows(head_dim: int) -> Optional[int]:
-    """Queries per tile of the second list the prefill attention takes for long portions (the kernel
-    that walks two 128-query tiles a block, csrc/attention_prefill_tc5.cu), or None for head sizes
-    it does not cover."""
-    return 256 if head_dim == 128 else None
+    """Queries per tile of the second list the prefill attention takes: for head size 128 the list of the kernel
+    that walks two 128-query tiles a block (long portions), for 256 that of the tcgen05 kernel, whose tiles are longer than the
+    mma.sync kernel's (csrc/attention_prefill_tc5.cu); None for other head sizes."""
+    return {128: 256, 256: 128}.get(head_dim)
 
 
 def _check_sinks(what: str, num_q_heads: int, sinks: Optional[torch.Tensor]) -> None:
@@ -971,7 +971,8 @@ def attention_prefill_mma(
 
     ``wide_tiles`` (count, rows, starts of tiles of ``attention_prefill_wide_tile_rows`` queries over the
     same portions): long portions of head size 128 go to the kernel that takes two query tiles a block
-    when its grid makes two waves or more; ``two_tiles`` overrides that choice (tests).
+    when its grid makes two waves or more; ``two_tiles`` overrides that choice (tests).  Portions of head size 256 go to the tcgen05 kernel
+    with that list, and to the mma.sync kernel without.
 
     ``sinks``: fp32 [heads], a logit a head whose exp joins the softmax's denominator.  ``gate``: bf16 [tokens, >= heads *
     head_dim], columns laid out as ``out``'s; the result is multiplied by its sigmoid.  Every kernel here takes both, in its
@@ -986,7 +987,14 @@ def attention_prefill_mma(
     if not attention_mma_supported(head_dim, num_q_heads, num_kv_heads):
         raise KernelError(f"{what}: head_dim {head_dim} with {num_q_heads}/{num_kv_heads} heads is not supported")
     gate_by_16 = gate is None or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)  # the tcgen05 kernel reads it in 16-byte groups
-    if gate_by_16 and _prefill_tc5_ok(q, out, k_cache, v_cache):  # tcgen05 + TMA: S and O in tensor memory
+    tensor_memory = gate_by_16 and _prefill_tc5_ok(q, out, k_cache, v_cache)
+    if tensor_memory and head_dim == 256:
+        tensor_memory = wide_tiles is not None and wide_tiles[0] > 0
+        if tensor_memory:
+            num_tiles, tile_rows, tile_starts = wide_tiles
+            _need_cuda(what, tile_rows, tile_starts)
+            _need_i32(what, tile_rows, tile_starts)
+    if tensor_memory:  # tcgen05 + TMA: S and O in tensor memory
         fn = _fn(
             "attention_prefill_tc5",
             "kb_attention_prefill_tc5",
@@ -1139,7 +1147,7 @@ def attention_decode_mma(
 def _prefill_tc5_ok(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
     head_dim = k_cache.shape[3]
     return (
-        head_dim in (64, 128)
+        head_dim in (64, 128, 256)
         and _decode_tma_ok(k_cache, v_cache)
         and q.stride(1) == 1 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
         and out.stride(1) == 1 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
