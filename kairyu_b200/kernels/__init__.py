@@ -9,6 +9,7 @@ an error.  Model parts call these as ``kernels.<name>(...)``.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from dataclasses import dataclass
 from typing import Optional
@@ -785,7 +786,13 @@ def _wide_row_map(cache: torch.Tensor) -> int:
     return (ctypes.addressof(held) + 63) & ~63
 
 
-DIFF_ATTENTION_TILE = 64  # queries a tile of the tensor-core kernel for prompt portions
+DIFF_ATTENTION_TILE = 64  # queries a tile of the mma.sync kernel for prompt portions
+DIFF_ATTENTION_TC5_TILE = 128  # ... of the tcgen05 kernel
+
+
+def diff_attention_tc5_supported(head_dim: int, value_dim: int) -> bool:
+    """Whether portions of such heads have a tcgen05 kernel (pages of a power of two from 8 up)."""
+    return head_dim in (64, 128) and value_dim in (64, 128)
 
 
 DIFF_ATTENTION_MMA_MAPS = (2,)  # how many softmax maps a head the tensor-core kernel is built for
@@ -818,7 +825,8 @@ def diff_attention_mma(
 ) -> None:
     """``diff_attention_generic`` on tensor cores (bfloat16, two maps): the step's prompt portions go tile by
     tile (``ctx.tiles[DIFF_ATTENTION_TILE]``), its single-token rows a key/value head at a time
-    (``ctx.decode_rows``), in two launches of one kernel.  ``ctx``: the step's description."""
+    (``ctx.decode_rows``).  Where the step lists tiles of ``DIFF_ATTENTION_TC5_TILE`` queries too, portions of sizes that kernel takes go to
+    tcgen05 (csrc/diff_attention_tc5.cu).  ``ctx``: the step's description."""
     what = "diff_attention_mma"
     _need_cuda(what, q, out, k_cache, v_cache, block_table, flag)
     _need_i32(what, block_table)
@@ -836,7 +844,23 @@ def diff_attention_mma(
                   0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0), float(out_scale), _ptr(flag), _stream()), what)
 
     num_tiles, tile_rows, tile_starts = ctx.tiles[DIFF_ATTENTION_TILE]
-    if num_tiles:
+    long_tiles = ctx.tiles.get(DIFF_ATTENTION_TC5_TILE)
+    if num_tiles and long_tiles is not None and scale > 0.0 and diff_attention_tc5_supported(dim, vdim) and page_size >= 8 and page_size & (page_size - 1) == 0 \
+            and all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in (q, out, k_cache, v_cache)):
+        num_tiles, tile_rows, tile_starts = long_tiles
+        _need_i32(what, tile_rows, tile_starts)
+        cap, near = None, 0.0
+        if softcap > 0.0:
+            near = SOFTCAP_NEAR_LIMIT * softcap / scale
+            cap = _both_caps(float(scale), float(softcap))
+        tc5 = _fn("diff_attention_tc5", "kb_diff_attention_tc5",
+                  [c_void_p] * 4 + [c_int] + [c_void_p] * 3 + [c_int] + [c_void_p] * 2 + [c_int] * 7 + [c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float, c_void_p, c_void_p])
+        merged = bool(_fn("diff_attention_tc5", "kb_diff_attention_tc5_merged", [c_int, c_int])(vdim, page_size))
+        _check(tc5(_tensor_map(q, 128), _cache_map(k_cache), _cache_map(v_cache, bands=merged), out.data_ptr(), out.stride(0), ctx.qo_indptr.data_ptr(),
+                   ctx.seq_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], tile_rows.data_ptr(), tile_starts.data_ptr(), int(num_tiles), num_q_heads,
+                   num_kv_heads, dim, vdim, page_size, num_pages, float(scale), int(window), float(lam), 0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0),
+                   float(out_scale), _softcap_address(cap), near, _ptr(flag), _stream()), what)
+    elif num_tiles:
         launch(tile_rows, tile_starts, num_tiles, 0)
     if ctx.num_decode_rows:
         launch(ctx.decode_rows, ctx.decode_tokens, ctx.num_decode_rows, 1)
@@ -879,6 +903,12 @@ class SoftCap(ctypes.Structure):
     @property
     def address(self) -> int:
         return ctypes.addressof(self)
+
+
+@functools.lru_cache(maxsize=256)
+def _both_caps(scale: float, cap: float) -> SoftCap:
+    """A cap with the coefficients of both forms, the near one fitted to all it covers: a kernel that looks at the scores chooses."""
+    return SoftCap.make(scale, cap, SOFTCAP_NEAR_LIMIT * cap / scale * (1.0 - 1e-9))
 
 
 def _softcap_address(softcap: Optional[SoftCap]) -> Optional[int]:

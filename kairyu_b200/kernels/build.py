@@ -33,6 +33,7 @@ LIBRARIES: dict[str, list[str]] = {
     "attention_generic": [],
     "diff_attention": [],
     "diff_attention_mma": [],
+    "diff_attention_tc5": [],
     "attention_mma": [],
     "attention_decode_static": [],
     "attention_decode_tma": [],

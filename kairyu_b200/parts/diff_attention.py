@@ -126,7 +126,10 @@ class DifferentialAttention(Mixer):
         return self.dtype == torch.bfloat16 and kernels.diff_attention_mma_supported(self.head_dim, self.value_dim, self.num_heads, self.num_kv_heads)
 
     def query_tile_sizes(self) -> tuple[int, ...]:
-        return (kernels.DIFF_ATTENTION_TILE,) if self._tensor_cores() else ()
+        if not self._tensor_cores():
+            return ()
+        tc5 = kernels.diff_attention_tc5_supported(self.head_dim, self.value_dim)
+        return (kernels.DIFF_ATTENTION_TILE,) + ((kernels.DIFF_ATTENTION_TC5_TILE,) if tc5 else ())
 
     # -- compute
     def fusable_norm(self, tokens: int) -> bool:
