@@ -535,11 +535,22 @@ __global__ void gather_rows_kernel(const T* __restrict__ src, const int* __restr
     for (int i = threadIdx.x; i < H; i += blockDim.x) o[i] = s[i];
 }
 
+// The same in 16-byte groups (8,192 rows of 4 KB: 19 us in 2-byte ones)
+__global__ void gather_rows_wide_kernel(const uint4* __restrict__ src, const int* __restrict__ rows, uint4* __restrict__ out, int groups) {
+    pdl_wait();
+    const uint4* s = src + (size_t)rows[blockIdx.x] * groups;
+    uint4* o = out + (size_t)blockIdx.x * groups;
+    for (int i = threadIdx.x; i < groups; i += blockDim.x) o[i] = s[i];
+}
+
 KB_EXPORT int kb_gather_rows(const void* src, const int* rows, void* out, int is_bf16, int R, int H,
                              cudaStream_t stream) {
     if (R == 0) return 0;
     if (!src || !rows || !out) return KB_ERR_NULL;
-    if (is_bf16)
+    const int per = is_bf16 ? 8 : 4;
+    if (H % per == 0 && (((uintptr_t)src | (uintptr_t)out) & 15) == 0)
+        kb_launch(gather_rows_wide_kernel, dim3(R), dim3(H / per >= 256 ? 256 : 128), 0, stream, (const uint4*)src, rows, (uint4*)out, H / per);
+    else if (is_bf16)
         kb_launch(gather_rows_kernel<__nv_bfloat16>, dim3(R), dim3(256), 0, stream, (const __nv_bfloat16*)src, rows, (__nv_bfloat16*)out, H);
     else
         kb_launch(gather_rows_kernel<float>, dim3(R), dim3(256), 0, stream, (const float*)src, rows, (float*)out, H);

@@ -109,36 +109,73 @@ __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ ids, int pairs, int E, int top, int* __restrict__ sorted, int* __restrict__ token_of,
                 int* __restrict__ place_of, int* __restrict__ ends, int* __restrict__ tile_expert,
                 int* __restrict__ tile_first, int* __restrict__ tile_pairs, int* __restrict__ num_tiles) {
+    // A thread's pairs are read ahead, eight at a time, so that their latency is paid once and not once a pair; the runs' places come from a scan by the first
+    // warp (8,192 pairs of 32 experts: 15.4 us with both in turn).
+    constexpr int AHEAD = 8;
     __shared__ int counts[MOE_MAX_EXPERTS];
     __shared__ int cursor[MOE_MAX_EXPERTS];
     pdl_wait();
     for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&counts[ids[p]], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0, tiles = 0;
-        for (int e = 0; e < E; ++e) {
-            cursor[e] = at;
-            for (int first = 0; first < counts[e]; first += MOE_TM) {
-                tile_expert[tiles] = e;
-                tile_first[tiles] = at + first;
-                tile_pairs[tiles] = min(MOE_TM, counts[e] - first);
-                ++tiles;
-            }
-            at += counts[e];
-            ends[e] = at;
+    int id[AHEAD];
+    auto fetch = [&](int p0) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int p = p0 + i * blockDim.x + threadIdx.x;
+            id[i] = p < pairs ? ids[p] : -1;
         }
-        *num_tiles = tiles;
+    };
+    for (int p0 = 0; p0 < pairs; p0 += AHEAD * blockDim.x) {
+        fetch(p0);
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (id[i] >= 0) atomicAdd(&counts[id[i]], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int at = 0, tiles = 0;  // pairs and tiles of the experts before
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, count = e < E ? counts[e] : 0, mine = (count + MOE_TM - 1) / MOE_TM;
+            int pairs_upto = count, tiles_upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int p = __shfl_up_sync(0xffffffffu, pairs_upto, o), t = __shfl_up_sync(0xffffffffu, tiles_upto, o);
+                if (lane >= o) {
+                    pairs_upto += p;
+                    tiles_upto += t;
+                }
+            }
+            const int start = at + pairs_upto - count;
+            if (e < E) {
+                cursor[e] = start;
+                ends[e] = start + count;
+            }
+            for (int i = 0; i < mine; ++i) {
+                const int tile = tiles + tiles_upto - mine + i;
+                tile_expert[tile] = e;
+                tile_first[tile] = start + i * MOE_TM;
+                tile_pairs[tile] = min(MOE_TM, count - i * MOE_TM);
+            }
+            at += __shfl_sync(0xffffffffu, pairs_upto, 31);
+            tiles += __shfl_sync(0xffffffffu, tiles_upto, 31);
+        }
+        if (lane == 0) *num_tiles = tiles;
     }
     __syncthreads();
     // The order of the pairs inside an expert's run is whatever the additions below give; a pair's
     // result does not depend on its place in a tile.
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int place = atomicAdd(&cursor[ids[p]], 1);
-        sorted[place] = p;
-        token_of[place] = p / top;
-        place_of[p] = place;
+    for (int p0 = 0; p0 < pairs; p0 += AHEAD * blockDim.x) {
+        if (pairs > AHEAD * (int)blockDim.x) fetch(p0);  // else they are still here
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            if (id[i] < 0) continue;
+            const int p = p0 + i * blockDim.x + threadIdx.x;
+            const int place = atomicAdd(&cursor[id[i]], 1);
+            sorted[place] = p;
+            token_of[place] = p / top;
+            place_of[p] = place;
+        }
     }
 }
 
@@ -151,6 +188,48 @@ moe_activation_kernel(const T* __restrict__ gate_up, T* __restrict__ y, int F, f
     const size_t row = i / F, col = i % F;
     const float gate = to_float(gate_up[row * 2 * F + col]), up = to_float(gate_up[row * 2 * F + F + col]);
     y[i] = from_float<T>(expert_activation(gate, up, limit, alpha, shift));
+}
+
+// Eight bfloat16 of a row at once
+struct Eight {
+    float v[8];
+    __device__ __forceinline__ void load(const __nv_bfloat16* at) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(at);
+        const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 two = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&words[i]));
+            v[2 * i] = two.x, v[2 * i + 1] = two.y;
+        }
+    }
+    __device__ __forceinline__ void load(const float* at) {
+        const float4 a = *reinterpret_cast<const float4*>(at), b = *reinterpret_cast<const float4*>(at + 4);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    }
+    __device__ __forceinline__ void store(__nv_bfloat16* at) const {
+        uint32_t words[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            words[i] = *reinterpret_cast<uint32_t*>(&two);
+        }
+        *reinterpret_cast<uint4*>(at) = make_uint4(words[0], words[1], words[2], words[3]);
+    }
+};
+
+// The same for bfloat16 rows of whole 16-byte groups, eight columns a thread (8,192 pairs of 1,024 columns: 34 us with one).
+__global__ void __launch_bounds__(256)
+moe_activation_wide_kernel(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ y, int F, float limit, float alpha, float shift, size_t groups) {
+    pdl_wait();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= groups) return;
+    const size_t row = i / (F / 8), col = i % (F / 8) * 8;
+    Eight gate, up;
+    gate.load(gate_up + row * 2 * F + col);
+    up.load(gate_up + row * 2 * F + F + col);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) gate.v[e] = expert_activation(gate.v[e], up.v[e], limit, alpha, shift);
+    gate.store(y + i * 8);
 }
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -354,18 +433,23 @@ moe_grouped_kernel(const T* __restrict__ A, int lda, const int* __restrict__ sor
 // from global memory (a row gives 128 contiguous bytes per step) and 16 bytes of its pair's row from shared
 // memory; the sum over k is taken in a permuted order that both operands share (columns tg*8+4j+{0..3} of a
 // 32-column run feed the j-th mma), so no data is shuffled.  The next step's loads are issued before this
-// step's products.  More than 8 pairs of a tile go in turns of 8 (the weights come from the L2 the second time).
+// step's products, and the first step's before the pairs' rows are staged.  The second product's rows are short, so a block's second four warps take the
+// second half of its columns and the halves' sums meet in shared memory (32 pairs of 19 of 32 experts, 1,024 columns: 23.8 -> 22.4 us; the first product,
+// with both halves of 2,048 columns streaming at once, goes from 41.6 to 48.3 and stays whole).  More than 8 pairs of a tile go in turns of 8 (the weights
+// come from the L2 the second time).
 #define SK_PAIRS 8
 #define SK_FEATURES 64
+__host__ __device__ constexpr int sk_parts(int form) { return form == MOE_DOWN ? 2 : 1; }
 
 template <int FORM>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128 * sk_parts(FORM))
 moe_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __restrict__ sorted, int top,
                   const __nv_bfloat16* __restrict__ W, int N, int Kd, int Kp, const int* __restrict__ tile_expert,
                   const int* __restrict__ tile_first, const int* __restrict__ tile_pairs, const int* __restrict__ num_tiles,
                   float limit, float alpha, float shift, int real_experts, void* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char sk_shared[];
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(sk_shared);  // [SK_PAIRS][Kp + 32]
+    constexpr int PARTS = sk_parts(FORM);
     constexpr bool FIRST = FORM != MOE_DOWN;
     constexpr int NB = FORM == MOE_GATED ? 2 : 1;
     // runs of 32 columns a step: one weight instead of two a lane leaves registers (and needs loads in flight) for twice the run
@@ -376,8 +460,9 @@ moe_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __res
     if (tile >= *num_tiles) return;
     const int expert = tile_expert[tile], first = tile_first[tile], rows = tile_pairs[tile];
     if (expert >= real_experts) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (threadIdx.x >> 5) & 3, part = threadIdx.x >> 7, lane = threadIdx.x & 31;
     const int g = lane >> 2, tg = lane & 3;
+    const int k_mid = PARTS == 1 ? Kp : (Kp / STEP + 1) / 2 * STEP, k_begin = part ? k_mid : 0, k_end = part ? Kp : k_mid;  // this part's columns
     const int f0 = blockIdx.y * SK_FEATURES + warp * 16;
     const int r0 = f0 + g, r1 = f0 + g + 8;
     const __nv_bfloat16* We = W + (size_t)expert * NB * N * Kd;
@@ -390,8 +475,22 @@ moe_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __res
         w1[b] = We + ((size_t)b * N + (r1 < N ? r1 : 0)) * Kd;
     }
     const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+    float* halves = reinterpret_cast<float*>(sk_shared + (size_t)SK_PAIRS * ldx * sizeof(__nv_bfloat16));  // [warp][NB * 4][lane]
+    uint4 lo[NB][RUNS], hi[NB][RUNS], nlo[NB][RUNS], nhi[NB][RUNS];
+    auto fetch = [&](int kc, uint4 (&dlo)[NB][RUNS], uint4 (&dhi)[NB][RUNS]) {
+#pragma unroll
+        for (int half = 0; half < RUNS; ++half) {
+            const int col = kc + half * 32 + tg * 8;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                dlo[b][half] = col < Kd ? __ldg(reinterpret_cast<const uint4*>(w0[b] + col)) : zero4;
+                dhi[b][half] = col < Kd ? __ldg(reinterpret_cast<const uint4*>(w1[b] + col)) : zero4;
+            }
+        }
+    };
     for (int sub = 0; sub < rows; sub += SK_PAIRS) {
         const int np = min(SK_PAIRS, rows - sub);
+        fetch(k_begin, lo, hi);
         __syncthreads();
         for (int idx = threadIdx.x; idx < SK_PAIRS * (Kp / 8); idx += blockDim.x) {
             const int i = idx / (Kp / 8), c = (idx % (Kp / 8)) * 8;
@@ -409,21 +508,8 @@ moe_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __res
         for (int b = 0; b < NB; ++b)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[b][c] = 0.0f;
-        uint4 lo[NB][RUNS], hi[NB][RUNS], nlo[NB][RUNS], nhi[NB][RUNS];
-        auto fetch = [&](int kc, uint4 (&dlo)[NB][RUNS], uint4 (&dhi)[NB][RUNS]) {
-#pragma unroll
-            for (int half = 0; half < RUNS; ++half) {
-                const int col = kc + half * 32 + tg * 8;
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    dlo[b][half] = col < Kd ? __ldg(reinterpret_cast<const uint4*>(w0[b] + col)) : zero4;
-                    dhi[b][half] = col < Kd ? __ldg(reinterpret_cast<const uint4*>(w1[b] + col)) : zero4;
-                }
-            }
-        };
-        fetch(0, lo, hi);
-        for (int kc = 0; kc < Kp; kc += STEP) {
-            if (kc + STEP < Kp) fetch(kc + STEP, nlo, nhi);
+        for (int kc = k_begin; kc < k_end; kc += STEP) {
+            if (kc + STEP < k_end) fetch(kc + STEP, nlo, nhi);
 #pragma unroll
             for (int half = 0; half < RUNS; ++half) {
                 const uint4 x = *reinterpret_cast<const uint4*>(xs + (size_t)g * ldx + kc + half * 32 + tg * 8);
@@ -436,7 +522,7 @@ moe_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __res
                     mma_bf16_16816(acc[b], a1, b1);
                 }
             }
-            if (kc + STEP < Kp) {
+            if (kc + STEP < k_end) {
 #pragma unroll
                 for (int b = 0; b < NB; ++b)
 #pragma unroll
@@ -445,6 +531,20 @@ moe_skinny_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __res
                         hi[b][half] = nhi[b][half];
                     }
             }
+        }
+        if constexpr (PARTS == 2) {
+            if (part == 1) {
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) halves[((warp * NB + b) * 4 + c) * 32 + lane] = acc[b][c];
+            }
+            __syncthreads();
+            if (part == 1) continue;
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[b][c] += halves[((warp * NB + b) * 4 + c) * 32 + lane];
         }
         // lane (g, tg) holds features r0 (c 0, 1) and r1 (c 2, 3) of pairs 2 tg and 2 tg + 1
 #pragma unroll
@@ -484,6 +584,44 @@ moe_combine_kernel(const TR* __restrict__ rows, const float* __restrict__ weight
         }
         if (extra) v += extra_weight * to_float(extra[(size_t)t * H + i]);
         out[(size_t)t * H + i] = from_float<TO>(v);
+    }
+}
+
+// The same for rows of whole groups of eight columns, eight a thread; the pairs of a token are looked up once a block (2,048 tokens of 2,048 columns: 18 us with one).
+template <typename TR, typename TO>
+__global__ void __launch_bounds__(256)
+moe_combine_wide_kernel(const TR* __restrict__ rows, const float* __restrict__ weights, const int* __restrict__ at, int K, int H,
+                        TO* __restrict__ out, const int* __restrict__ ids, const TO* __restrict__ x, int real_experts,
+                        const TO* __restrict__ extra, const float* __restrict__ extra_gate, int gate_stride) {
+    __shared__ float weight[MOE_MAX_TOP];
+    __shared__ long long place[MOE_MAX_TOP];  // -1: an identity expert, whose output is the token's own row
+    const int t = blockIdx.x;
+    pdl_wait();
+    if (threadIdx.x < K) {
+        const size_t p = (size_t)t * K + threadIdx.x;
+        weight[threadIdx.x] = weights ? weights[p] : 1.0f;
+        place[threadIdx.x] = ids && ids[p] >= real_experts ? -1 : at ? (long long)at[p] : (long long)p;
+    }
+    __syncthreads();
+    const float extra_weight = extra ? (extra_gate ? 1.0f / (1.0f + expf(-extra_gate[(size_t)t * gate_stride])) : 1.0f) : 0.0f;
+    for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
+        Eight sum, row;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sum.v[e] = 0.0f;
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            if (place[k] < 0) row.load(x + (size_t)t * H + i);
+            else row.load(rows + (size_t)place[k] * H + i);
+            const float w = weight[k];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum.v[e] += w * row.v[e];
+        }
+        if (extra) {
+            row.load(extra + (size_t)t * H + i);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum.v[e] += extra_weight * row.v[e];
+        }
+        sum.store(out + (size_t)t * H + i);
     }
 }
 
@@ -647,7 +785,9 @@ KB_EXPORT int kb_moe_activation(const void* gate_up, void* y, int is_bf16, int r
     if (!gate_up || !y) return KB_ERR_NULL;
     const size_t total = (size_t)rows * F;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (is_bf16)
+    if (is_bf16 && F % 8 == 0 && (((uintptr_t)gate_up | (uintptr_t)y) & 15) == 0)
+        kb_launch(moe_activation_wide_kernel, dim3((unsigned)((total / 8 + 255) / 256)), dim3(256), 0, stream, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)y, F, limit, alpha, shift, total / 8);
+    else if (is_bf16)
         kb_launch(moe_activation_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)y, F, limit, alpha, shift, total);
     else
         kb_launch(moe_activation_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)gate_up, (float*)y, F, limit, alpha, shift, total);
@@ -684,13 +824,13 @@ KB_EXPORT int kb_moe_skinny(const void* A, int lda, const int* sorted, int top, 
     if (N < 1 || Kd < 8 || top < 1 || Kd % 8 != 0 || lda % 8 != 0 || ((uintptr_t)A % 16) != 0 || ((uintptr_t)W % 16) != 0) return KB_ERR_BAD_ARG;
     const int step = form == MOE_GATED ? 64 : 128;  // the kernel's columns a step
     const int Kp = (Kd + step - 1) / step * step;
-    const size_t smem = (size_t)SK_PAIRS * (Kp + 32) * sizeof(__nv_bfloat16);
+    const size_t smem = (size_t)SK_PAIRS * (Kp + 32) * sizeof(__nv_bfloat16) + (sk_parts(form) == 2 ? 4 * 4 * 32 * sizeof(float) : 0);
     if (smem > 200 * 1024) return KB_ERR_UNSUPPORTED_SIZE;
     dim3 grid(max_tiles, (N + SK_FEATURES - 1) / SK_FEATURES);
 #define LAUNCH(F)                                                                                                                             \
     do {                                                                                                                                      \
         if (smem > 48 * 1024) cudaFuncSetAttribute(moe_skinny_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-        kb_launch(moe_skinny_kernel<F>, grid, dim3(128), smem, stream, (const __nv_bfloat16*)A, lda, sorted, top, (const __nv_bfloat16*)W, N, Kd, \
+        kb_launch(moe_skinny_kernel<F>, grid, dim3(128 * sk_parts(F)), smem, stream, (const __nv_bfloat16*)A, lda, sorted, top, (const __nv_bfloat16*)W, N, Kd, \
                   Kp, tile_expert, tile_first, tile_pairs, num_tiles, limit, alpha, shift, real_experts, out);                                  \
     } while (0)
     if (form == MOE_GATED) LAUNCH(MOE_GATED);
@@ -705,6 +845,16 @@ KB_EXPORT int kb_moe_combine(const void* rows, int rows_is_bf16, const float* we
                              const float* extra_gate, int gate_stride, cudaStream_t stream) {
     if (T == 0) return 0;
     if (!rows || !out || (ids && !x)) return KB_ERR_NULL;
+    if (out_is_bf16 && H % 8 == 0 && K <= MOE_MAX_TOP && (((uintptr_t)rows | (uintptr_t)out | (uintptr_t)x | (uintptr_t)extra) & 15) == 0) {
+        const dim3 block(H >= 2048 ? 256 : H >= 1024 ? 128 : 64);
+        if (rows_is_bf16)
+            kb_launch(moe_combine_wide_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(T), block, 0, stream, (const __nv_bfloat16*)rows, weights, at, K, H, (__nv_bfloat16*)out, ids,
+                      (const __nv_bfloat16*)x, real_experts, (const __nv_bfloat16*)extra, extra_gate, gate_stride);
+        else
+            kb_launch(moe_combine_wide_kernel<float, __nv_bfloat16>, dim3(T), block, 0, stream, (const float*)rows, weights, at, K, H, (__nv_bfloat16*)out, ids,
+                      (const __nv_bfloat16*)x, real_experts, (const __nv_bfloat16*)extra, extra_gate, gate_stride);
+        return kb_launch_result();
+    }
 #define LAUNCH(TR, TO)                                                                                                     \
     kb_launch(moe_combine_kernel<TR, TO>, dim3(T), dim3(256), 0, stream, (const TR*)rows, weights, at, K, H, (TO*)out, ids, \
               (const TO*)x, real_experts, (const TO*)extra, extra_gate, gate_stride)
