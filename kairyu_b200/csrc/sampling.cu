@@ -107,11 +107,13 @@ KB_EXPORT int kb_argmax(const float* logits, int ld, int n, int V, int* out, cud
 //
 // Two launches.  The first cuts a row into chunks (32 of them, or more for a vocabulary beyond
 // 262,144) with a block each: the chunk's part of the log-sum-exp (running maximum, sum) and its own
-// k best entries, found by k passes over the chunk, which the L1 holds after the first.  Pass i finds
+// k best entries, found by k passes over the chunk, which the block's registers hold.  Pass i finds
 // the best entry that comes after pass i-1's in the order (value down, index up), so nothing has to
 // be remembered but the last.  The second launch, a block a report, adds the chunks' sums in chunk
 // order and finds the k best among the chunks' candidates the same way.  (One block a row, k + 1
-// passes over the whole row, took 250 us at 128,256 entries and k = 5.)
+// passes over the whole row, took 250 us at 128,256 entries and k = 5.)  Both wait for memory and block
+// meetings, not bandwidth: with the chunk read again by each pass and one thread fetching the chunks' sums
+// one behind the other they took 16 and 10 us at eight reports of 128,256 entries; now 12.0 and 7.9.
 constexpr int REPORT_THREADS = 256;
 constexpr int REPORT_WARPS = REPORT_THREADS / 32;
 constexpr int REPORT_CHUNKS = 32;
@@ -149,7 +151,9 @@ __device__ void report_block_best(float& best, int& best_i, float* red_v, int* r
         if (report_before(red_v[w], red_i[w], best, best_i)) { best = red_v[w]; best_i = red_i[w]; }
 }
 
-// grid (reports, chunks)
+// grid (reports, chunks).  PER: the entries a thread holds in registers, chunk_len <= PER * REPORT_THREADS, so that
+// they are all asked for at once and the k passes read no memory.
+template <int PER>
 __global__ void __launch_bounds__(REPORT_THREADS)
 logprob_chunk_kernel(const float* __restrict__ logits, int ld, int V, const int* __restrict__ rows, int k, int chunk_len,
                      float* __restrict__ scratch) {
@@ -165,10 +169,17 @@ logprob_chunk_kernel(const float* __restrict__ logits, int ld, int V, const int*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* mine = scratch + ((size_t)r * gridDim.y + chunk) * report_scratch_floats(k);
 
+    float held[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int i = begin + threadIdx.x + j * REPORT_THREADS;
+        held[j] = i < end ? x[i] : -INFINITY;
+    }
     // the chunk's part of the log of the sum of exponentials, with the running maximum taken out
     float m = -INFINITY, sum = 0.0f;
-    for (int i = begin + threadIdx.x; i < end; i += REPORT_THREADS) {
-        const float v = x[i];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const float v = held[j];  // past the end: -inf, which adds nothing
         if (v > m) {
             sum = sum * expf(m - v) + 1.0f;  // m = -inf: sum is 0 and stays finite
             m = v;
@@ -202,12 +213,15 @@ logprob_chunk_kernel(const float* __restrict__ logits, int ld, int V, const int*
     for (int pass = 0; pass < k; ++pass) {
         float best = -INFINITY;
         int best_i = REPORT_ABSENT;
-        if (prev_i != REPORT_ABSENT)  // else nothing is left: later passes find nothing either
-            for (int i = begin + threadIdx.x; i < end; i += REPORT_THREADS) {
-                const float v = x[i];
-                const bool after = v < prev_v || (v == prev_v && i > prev_i);
+        if (prev_i != REPORT_ABSENT) {  // else nothing is left: later passes find nothing either
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                const int i = begin + threadIdx.x + j * REPORT_THREADS;
+                const float v = held[j];
+                const bool after = i < end && (v < prev_v || (v == prev_v && i > prev_i));
                 if (after && report_before(v, i, best, best_i)) { best = v; best_i = i; }
             }
+        }
         report_block_best(best, best_i, red_m, red_i);
         if (threadIdx.x == 0) {
             mine[2 + 2 * pass] = best;
@@ -232,14 +246,32 @@ logprob_merge_kernel(const float* __restrict__ logits, int ld, int V, const int*
     const float* x = logits + (size_t)row * ld;
     const size_t per = report_scratch_floats(k);
     const float* mine = scratch + (size_t)r * chunks * per;
-    if (threadIdx.x == 0) {
-        float bm = mine[0], bs = mine[1];
-        for (int c = 1; c < chunks; ++c) {  // in chunk order
-            const float cm = mine[c * per], cs = mine[c * per + 1];
-            const float nm = fmaxf(bm, cm);
-            if (nm > -INFINITY) bs = bs * expf(bm - nm) + cs * expf(cm - nm);
-            bm = nm;
+    // the chunks' sums come in together, a block's width of them at a time; one thread adds them in chunk order
+    __shared__ float chunk_m[REPORT_THREADS], chunk_s[REPORT_THREADS];
+    float bm = -INFINITY, bs = 0.0f;
+    for (int c0 = 0; c0 < chunks; c0 += REPORT_THREADS) {
+        const int count = min(REPORT_THREADS, chunks - c0);
+        if (threadIdx.x < count) {
+            chunk_m[threadIdx.x] = mine[(size_t)(c0 + threadIdx.x) * per];
+            chunk_s[threadIdx.x] = mine[(size_t)(c0 + threadIdx.x) * per + 1];
         }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int c = 0; c < count; ++c) {
+                const float cm = chunk_m[c], cs = chunk_s[c];
+                if (c0 + c == 0) {
+                    bm = cm;
+                    bs = cs;
+                    continue;
+                }
+                const float nm = fmaxf(bm, cm);
+                if (nm > -INFINITY) bs = bs * expf(bm - nm) + cs * expf(cm - nm);
+                bm = nm;
+            }
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
         const float lse = bm + logf(bs);
         bcast = lse;
         int token = tokens[tokens_by_row ? row : r];
@@ -295,7 +327,10 @@ KB_EXPORT int kb_logprob_report(const float* logits, int ld, int n_rows, int V, 
     const int len = report_chunk_len(V);
     const int chunks = (V + len - 1) / len;
     if (chunks > 65535) return KB_ERR_UNSUPPORTED_SIZE;
-    kb_launch(logprob_chunk_kernel, dim3(reports, chunks), dim3(REPORT_THREADS), 0, stream, logits, ld, V, rows, k, len, scratch);
+    // 16 entries a thread reach vocabularies of 131,072 in 32 chunks; longer chunks take up to 32
+    static_assert(REPORT_MAX_CHUNK <= 32 * REPORT_THREADS, "a chunk fits the registers of its block");
+    const auto chunk_kernel = len <= 16 * REPORT_THREADS ? logprob_chunk_kernel<16> : logprob_chunk_kernel<32>;
+    kb_launch(chunk_kernel, dim3(reports, chunks), dim3(REPORT_THREADS), 0, stream, logits, ld, V, rows, k, len, scratch);
     int rc = kb_launch_result();
     if (rc != 0) return rc;
     kb_launch(logprob_merge_kernel, dim3(reports), dim3(REPORT_THREADS), 0, stream, logits, ld, V, rows, tokens, tokens_by_row, k,
