@@ -835,13 +835,17 @@ def diff_attention_mma(
         raise KernelError(f"{what}: bfloat16, two maps, sizes as diff_attention_mma_supported says")
     fn = _fn("diff_attention_mma", "kb_diff_attention_mma",
              [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
-              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_void_p])
+              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float, c_void_p, c_void_p])
+    cap, near = None, 0.0
+    if softcap > 0.0 and scale > 0.0:
+        near = SOFTCAP_NEAR_LIMIT * softcap / scale
+        cap = _both_caps(float(scale), float(softcap))
 
     def launch(rows: torch.Tensor, second: torch.Tensor, count: int, single: int) -> None:
         _check(fn(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), ctx.qo_indptr.data_ptr(),
                   ctx.seq_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], rows.data_ptr(), second.data_ptr(), int(count), single,
                   num_q_heads, num_kv_heads, dim, vdim, page_size, num_pages, float(scale), float(softcap), int(window), float(lam),
-                  0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0), float(out_scale), _ptr(flag), _stream()), what)
+                  0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0), float(out_scale), _softcap_address(cap), near, _ptr(flag), _stream()), what)
 
     num_tiles, tile_rows, tile_starts = ctx.tiles[DIFF_ATTENTION_TILE]
     long_tiles = ctx.tiles.get(DIFF_ATTENTION_TC5_TILE)
@@ -849,10 +853,6 @@ def diff_attention_mma(
             and all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in (q, out, k_cache, v_cache)):
         num_tiles, tile_rows, tile_starts = long_tiles
         _need_i32(what, tile_rows, tile_starts)
-        cap, near = None, 0.0
-        if softcap > 0.0:
-            near = SOFTCAP_NEAR_LIMIT * softcap / scale
-            cap = _both_caps(float(scale), float(softcap))
         tc5 = _fn("diff_attention_tc5", "kb_diff_attention_tc5",
                   [c_void_p] * 4 + [c_int] + [c_void_p] * 3 + [c_int] + [c_void_p] * 2 + [c_int] * 7 + [c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float, c_void_p, c_void_p])
         merged = bool(_fn("diff_attention_tc5", "kb_diff_attention_tc5_merged", [c_int, c_int])(vdim, page_size))
