@@ -398,6 +398,11 @@ KB_EXPORT int kb_diff_attention_tc5_supported(int D, int DV, int page_size) {
 // 1 where the map of the values has every 64-column band in a box (kb_attention_encode_cache_map with bands = 1)
 KB_EXPORT int kb_diff_attention_tc5_merged(int DV, int page_size) { return DV > 64 && page_size >= 16; }
 
+template <int KD, int KV>
+struct Sizes {
+    static constexpr int D = KD, DV = KV;
+};
+
 // map_q: 2-D map over the packed query rows [tokens, q_stride] with boxes of [128 rows, 64 columns]; map_k, map_v: maps over the caches as
 // kb_attention_prefill_tc5 takes them (a key row: both maps, 2 D columns).  The list holds 128 queries a tile.  softcap (optional): a host KbSoftcap with the
 // coefficients of both forms; near_limit: the largest |raw score| that its near form covers.
@@ -412,13 +417,18 @@ KB_EXPORT int kb_diff_attention_tc5(const void* map_q, const void* map_k, const 
     int shift = 0;
     while ((1 << shift) < page_size) ++shift;
     const KbSoftcap cap = kb_softcap_of(softcap);
-    auto launch = [&](auto kernel, size_t smem) {
-        if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return (int)e;
-        kb_launch(kernel, dim3(Hq, num_tiles), dim3(THREADS), smem, stream, *(const CUtensorMap*)map_q, *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v,
-                  (__nv_bfloat16*)out, out_stride, qo_indptr, seq_lens, block_table, max_pages, tile_rows, tile_starts, num_tiles, Hq, Hkv, page_size, shift, num_pages,
-                  scale, window, kb_diff_attention_tc5_merged(DV, page_size), lambda, head_norm, eps, out_scale, cap, near_limit, flag);
+    auto launch = [&](auto sizes) {
+        constexpr int KD = decltype(sizes)::D, KV = decltype(sizes)::DV;
+        static bool configured = false;  // of this pair of sizes
+        if (!configured) {
+            if (cudaError_t e = cudaFuncSetAttribute(diff_attention_tc5_kernel<KD, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<KD, KV>::SMEM)) return (int)e;
+            configured = true;
+        }
+        kb_launch(diff_attention_tc5_kernel<KD, KV>, dim3(Hq, num_tiles), dim3(THREADS), Cfg<KD, KV>::SMEM, stream, *(const CUtensorMap*)map_q, *(const CUtensorMap*)map_k,
+                  *(const CUtensorMap*)map_v, (__nv_bfloat16*)out, out_stride, qo_indptr, seq_lens, block_table, max_pages, tile_rows, tile_starts, num_tiles, Hq, Hkv,
+                  page_size, shift, num_pages, scale, window, kb_diff_attention_tc5_merged(DV, page_size), lambda, head_norm, eps, out_scale, cap, near_limit, flag);
         return kb_launch_result();
     };
-    if (D == 64) return DV == 64 ? launch(diff_attention_tc5_kernel<64, 64>, Cfg<64, 64>::SMEM) : launch(diff_attention_tc5_kernel<64, 128>, Cfg<64, 128>::SMEM);
-    return DV == 64 ? launch(diff_attention_tc5_kernel<128, 64>, Cfg<128, 64>::SMEM) : launch(diff_attention_tc5_kernel<128, 128>, Cfg<128, 128>::SMEM);
+    if (D == 64) return DV == 64 ? launch(Sizes<64, 64>{}) : launch(Sizes<64, 128>{});
+    return DV == 64 ? launch(Sizes<128, 64>{}) : launch(Sizes<128, 128>{});
 }

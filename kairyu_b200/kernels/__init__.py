@@ -788,6 +788,13 @@ def _wide_row_map(cache: torch.Tensor) -> int:
 
 DIFF_ATTENTION_TILE = 64  # queries a tile of the mma.sync kernel for prompt portions
 DIFF_ATTENTION_TC5_TILE = 128  # ... of the tcgen05 kernel
+# Sequences of one tile of keys stay on mma.sync: the tcgen05 kernel's set-up isn't made up for, and with more blocks than SMs (one an SM) it is paid once a
+# wave (us, both kernels: prompts of 9 to 50 tokens, eight of 32 heads: 18.2 against mma.sync's 12.7; in one wave 9.5 against 10.9, less than its
+# three tensor maps cost the host).  So do sequences of up to 192 keys whose mma.sync blocks run at once, two an SM: 11 against 17 at 100 tokens, but a call of
+# a layer that short waits for the host, 58 us against 51.  Beyond either line tcgen05 is ahead (one prompt of 400: 18.8 against 53; eight of up to 116, 32 heads:
+# 21.5 against 31.9).
+DIFF_ATTENTION_SHORT_KEYS = 64
+DIFF_ATTENTION_FEW_KEYS = 192
 
 
 def diff_attention_tc5_supported(head_dim: int, value_dim: int) -> bool:
@@ -803,6 +810,23 @@ def diff_attention_mma_supported(head_dim: int, value_dim: int, num_q_heads: int
     up to 128, up to 64 query heads a key/value head); others use the 32-bit-arithmetic kernel."""
     return (maps in DIFF_ATTENTION_MMA_MAPS and head_dim % 16 == 0 and 16 <= head_dim <= 128 and value_dim % 16 == 0 and 16 <= value_dim <= 128
             and num_kv_heads >= 1 and num_q_heads % num_kv_heads == 0 and num_q_heads // num_kv_heads <= 64)
+
+
+_DIFF_ATTENTION_MMA_ARGS = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
+                            c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float, c_void_p, c_void_p]
+_DIFF_ATTENTION_TC5_ARGS = [c_void_p] * 4 + [c_int] + [c_void_p] * 3 + [c_int] + [c_void_p] * 2 + [c_int] * 7 + [c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float,
+                                                                                                       c_void_p, c_void_p]
+
+
+@functools.lru_cache(maxsize=64)
+def _sm_count(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+@functools.lru_cache(maxsize=64)
+def _diff_tc5_merged(value_dim: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel fetches all of a value page's 64-column bands in one copy."""
+    return bool(_fn("diff_attention_tc5", "kb_diff_attention_tc5_merged", [c_int, c_int])(value_dim, page_size))
 
 
 def diff_attention_mma(
@@ -833,33 +857,33 @@ def diff_attention_mma(
     num_pages, page_size, num_kv_heads, dim, vdim = _check_diff_attention(what, q, out, k_cache, v_cache, num_q_heads, maps)
     if maps != 2 or q.dtype != torch.bfloat16 or k_cache.shape[2] != num_kv_heads or not diff_attention_mma_supported(dim, vdim, num_q_heads, num_kv_heads):
         raise KernelError(f"{what}: bfloat16, two maps, sizes as diff_attention_mma_supported says")
-    fn = _fn("diff_attention_mma", "kb_diff_attention_mma",
-             [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
-              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float, c_void_p, c_void_p])
-    cap, near = None, 0.0
-    if softcap > 0.0 and scale > 0.0:
-        near = SOFTCAP_NEAR_LIMIT * softcap / scale
-        cap = _both_caps(float(scale), float(softcap))
+    fn = _fn("diff_attention_mma", "kb_diff_attention_mma", _DIFF_ATTENTION_MMA_ARGS)
+    scale, softcap = float(scale), float(softcap)
+    held_cap, cap, near = _near_cap(scale, softcap)  # held until the launches below have copied it
+    q_at, out_at, k_at, v_at, q_step, out_step = q.data_ptr(), out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), q.stride(0), out.stride(0)
+    indptr_at, lens_at, table_at, table_width, flag_at, stream = ctx.qo_indptr.data_ptr(), ctx.seq_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], _ptr(flag), _stream()
+    head_norm, norm_eps = 0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0)
 
     def launch(rows: torch.Tensor, second: torch.Tensor, count: int, single: int) -> None:
-        _check(fn(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), ctx.qo_indptr.data_ptr(),
-                  ctx.seq_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], rows.data_ptr(), second.data_ptr(), int(count), single,
-                  num_q_heads, num_kv_heads, dim, vdim, page_size, num_pages, float(scale), float(softcap), int(window), float(lam),
-                  0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0), float(out_scale), _softcap_address(cap), near, _ptr(flag), _stream()), what)
+        _check(fn(q_at, q_step, out_at, out_step, k_at, v_at, indptr_at, lens_at, table_at, table_width, rows.data_ptr(), second.data_ptr(), int(count), single,
+                  num_q_heads, num_kv_heads, dim, vdim, page_size, num_pages, scale, softcap, int(window), float(lam), head_norm, norm_eps, float(out_scale),
+                  cap, near, flag_at, stream), what)
 
     num_tiles, tile_rows, tile_starts = ctx.tiles[DIFF_ATTENTION_TILE]
     long_tiles = ctx.tiles.get(DIFF_ATTENTION_TC5_TILE)
+    most_keys = getattr(ctx, "max_portion_seq_len", 0)  # 0: not known
+    if long_tiles is not None and 0 < most_keys <= DIFF_ATTENTION_FEW_KEYS \
+            and (most_keys <= DIFF_ATTENTION_SHORT_KEYS or num_tiles * num_q_heads <= 2 * _sm_count(q.get_device())):
+        long_tiles = None
     if num_tiles and long_tiles is not None and scale > 0.0 and diff_attention_tc5_supported(dim, vdim) and page_size >= 8 and page_size & (page_size - 1) == 0 \
-            and all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in (q, out, k_cache, v_cache)):
+            and (q_at | out_at | k_at | v_at) % 16 == 0 and (q_step | out_step | k_cache.stride(0) | v_cache.stride(0)) % 8 == 0:
         num_tiles, tile_rows, tile_starts = long_tiles
         _need_i32(what, tile_rows, tile_starts)
-        tc5 = _fn("diff_attention_tc5", "kb_diff_attention_tc5",
-                  [c_void_p] * 4 + [c_int] + [c_void_p] * 3 + [c_int] + [c_void_p] * 2 + [c_int] * 7 + [c_float, c_int, c_float, c_int, c_float, c_float, c_void_p, c_float, c_void_p, c_void_p])
-        merged = bool(_fn("diff_attention_tc5", "kb_diff_attention_tc5_merged", [c_int, c_int])(vdim, page_size))
-        _check(tc5(_tensor_map(q, 128), _cache_map(k_cache), _cache_map(v_cache, bands=merged), out.data_ptr(), out.stride(0), ctx.qo_indptr.data_ptr(),
-                   ctx.seq_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], tile_rows.data_ptr(), tile_starts.data_ptr(), int(num_tiles), num_q_heads,
-                   num_kv_heads, dim, vdim, page_size, num_pages, float(scale), int(window), float(lam), 0 if head_norm_eps is None else 1, float(head_norm_eps or 0.0),
-                   float(out_scale), _softcap_address(cap), near, _ptr(flag), _stream()), what)
+        tc5 = _fn("diff_attention_tc5", "kb_diff_attention_tc5", _DIFF_ATTENTION_TC5_ARGS)
+        merged = _diff_tc5_merged(vdim, page_size)
+        _check(tc5(_tensor_map(q, 128), _cache_map(k_cache), _cache_map(v_cache, bands=merged), out_at, out_step, indptr_at, lens_at, table_at, table_width,
+                   tile_rows.data_ptr(), tile_starts.data_ptr(), int(num_tiles), num_q_heads, num_kv_heads, dim, vdim, page_size, num_pages, scale, int(window),
+                   float(lam), head_norm, norm_eps, float(out_scale), cap, near, flag_at, stream), what)
     elif num_tiles:
         launch(tile_rows, tile_starts, num_tiles, 0)
     if ctx.num_decode_rows:
@@ -909,6 +933,18 @@ class SoftCap(ctypes.Structure):
 def _both_caps(scale: float, cap: float) -> SoftCap:
     """A cap with the coefficients of both forms, the near one fitted to all it covers: a kernel that looks at the scores chooses."""
     return SoftCap.make(scale, cap, SOFTCAP_NEAR_LIMIT * cap / scale * (1.0 - 1e-9))
+
+
+@functools.lru_cache(maxsize=256)
+def _held_cap(scale: float, cap: float) -> tuple[SoftCap, int, float]:
+    held = _both_caps(scale, cap)
+    return held, held.address, SOFTCAP_NEAR_LIMIT * cap / scale
+
+
+def _near_cap(scale: float, cap: float) -> tuple[Optional[SoftCap], Optional[int], float]:
+    """A cap with both forms, its address and the largest |raw score| of its near one; (None, None, 0.0) without a cap.  The address is good as long as the
+    caller holds the structure."""
+    return _held_cap(scale, cap) if cap > 0.0 and scale > 0.0 else (None, None, 0.0)
 
 
 def _softcap_address(softcap: Optional[SoftCap]) -> Optional[int]:

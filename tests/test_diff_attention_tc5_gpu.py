@@ -68,3 +68,32 @@ def test_portions(D, DV, heads, kv, page, counts, contexts, window, cap, spread,
         assert flag.item() == 0 and kernels.launch_count == before + 1
         # probabilities and the result rounded to 16 bits: 2^-8 of values of order one to four, and behind the norm of rows whose two maps nearly cancel a few times that
         assert (out.cpu().double().view_as(want) - want).abs().max() < 4e-2, sizes
+
+
+@pytest.mark.parametrize("rows,length,heads,short", [(8, 30, 32, True), (8, 64, 32, True), (8, 65, 32, False), (1, 192, 16, True), (1, 193, 16, False)])
+def test_short_portions_stay_on_mma_sync(rows, length, heads, short):
+    """Sequences of one key tile, and of up to 192 keys in few blocks: the same bits as a step that lists no tiles of 128; otherwise the same within rounding."""
+    from kairyu_b200 import kernels
+    from kairyu_b200.engine.workspace import Workspace
+
+    D = DV = 64
+    g = torch.Generator().manual_seed(rows + length)
+    k = torch.randn(13 * rows + 1, 16, 4, 2 * D, generator=g).bfloat16().cuda()
+    v = torch.randn(13 * rows + 1, 16, 4, DV, generator=g).bfloat16().cuda()
+    q = torch.randn(rows * length, heads * 2 * D, generator=g).bfloat16().cuda()
+    i32 = dict(dtype=torch.int32, device="cuda")
+
+    def tiles(size):
+        pairs = [(row, s) for row in range(rows) for s in range(0, length, size)]
+        return len(pairs), torch.tensor([row for row, _ in pairs], **i32), torch.tensor([s for _, s in pairs], **i32)
+
+    results = []
+    for sizes in ((kernels.DIFF_ATTENTION_TILE,), (kernels.DIFF_ATTENTION_TILE, kernels.DIFF_ATTENTION_TC5_TILE)):
+        ctx = types.SimpleNamespace(qo_indptr=torch.arange(0, rows * length + 1, length, **i32), seq_lens=torch.full((rows,), length, **i32), tiles={size: tiles(size) for size in sizes},
+                                    num_decode_rows=0, workspace=Workspace("cuda"), max_portion_seq_len=length)
+        out = torch.full((rows * length, heads * DV), float("nan"), dtype=torch.bfloat16, device="cuda")
+        kernels.diff_attention_mma(q, out, k, v, ctx=ctx, block_table=torch.arange(1, 13 * rows + 1, **i32).view(rows, 13), num_q_heads=heads, maps=2, scale=D ** -0.5, softcap=50.0,
+                                   lam=0.4)
+        results.append(out)
+    assert torch.equal(*results) == short
+    assert (results[0].float() - results[1].float()).abs().max() < 3e-2  # probabilities and results rounded to 16 bits, of values up to four
